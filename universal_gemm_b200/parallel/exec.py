@@ -21,6 +21,7 @@ fused executor.
 from __future__ import annotations
 
 import time
+import weakref
 from typing import Any, Sequence
 
 import torch
@@ -32,18 +33,34 @@ from . import tiles as T
 from .matrix import DistMatrix, resolve
 from .plan import MultiplyOp
 
+# Lowered programs by (kind, uids of the buffers of A, B, C, rank, fuse, beta, uid of the activation's buffer, number):
+# `number` counts the op lists that were lowered for the same matrices.  A program holds the addresses of all ranks'
+# tiles, so it is valid for the very allocations it was lowered for and lives no longer than the first of them.
 _program_cache: dict[tuple, Any] = {}
+_programs_of: dict[int, set[tuple]] = {}      # buffer uid -> its programs' keys
+_MAX_OP_LISTS = 8                             # op lists kept per matrix triple: the ninth takes the place of the eighth
 
 
 def clear_program_cache() -> None:
     _program_cache.clear()
+    for keys in list(_programs_of.values()):
+        keys.clear()
 
 
-def drop_programs_for(local_ptr: int) -> None:
-    """Forget lowered programs that reference the symmetric buffer at ``local_ptr`` (called when a matrix is
-    freed: a later allocation may get the same local address but different peer mappings)."""
-    for key in [k for k in _program_cache if local_ptr in k[1:4] or local_ptr == k[7]]:
-        del _program_cache[key]
+def drop_programs_for(uid: int) -> None:
+    """Forget the lowered programs of the symmetric buffer ``uid``, with their tables, staging area and workspace (called
+    when a matrix is freed, and when its buffer is collected)."""
+    for key in list(_programs_of.pop(uid, ())):
+        _program_cache.pop(key, None)
+
+
+def _keep_program(key: tuple, entry: tuple, buffers: Sequence[Any]) -> None:
+    for buf in buffers:
+        if buf.uid not in _programs_of:
+            _programs_of[buf.uid] = set()
+            weakref.finalize(buf, drop_programs_for, buf.uid).atexit = False
+        _programs_of[buf.uid].add(key)
+    _program_cache[key] = entry
 
 
 # ----------------------------------------------------------------------------- lowering
@@ -139,13 +156,17 @@ def lower_plan(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequ
 
 def _program(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequence[MultiplyOp], fuse: bool,
              beta: int = 1, gelu_out: DistMatrix | None = None):
-    act = gelu_out.buffer.ptr(c.rank) if gelu_out is not None else 0
-    key = (kind, a.buffer.ptr(a.rank), b.buffer.ptr(b.rank), c.buffer.ptr(c.rank), c.rank, fuse, beta, act)
-    hit = _program_cache.get(key)
-    if hit is not None and (hit[0] is ops or hit[0] == ops) and hit[1] == (a.layout, b.layout, c.layout):
-        return hit[2]
+    act = gelu_out.buffer.uid if gelu_out is not None else 0
+    form = (a.layout, b.layout, c.layout, a.dtype, b.dtype, c.dtype)
+    for number in range(_MAX_OP_LISTS):
+        key = (kind, a.buffer.uid, b.buffer.uid, c.buffer.uid, c.rank, fuse, beta, act, number)
+        hit = _program_cache.get(key)
+        if hit is None:
+            break
+        if (hit[0] is ops or hit[0] == ops) and hit[1] == form:
+            return hit[2]
     prog = lower_plan(kind, a, b, c, ops, fuse_replica_reduce=fuse, beta=beta, gelu_out=gelu_out)
-    _program_cache[key] = (ops, (a.layout, b.layout, c.layout), prog)
+    _keep_program(key, (ops, form, prog), [m.buffer for m in (a, b, c, gelu_out) if m is not None])
     trace.register(f"stationary_{kind} rank{c.rank} {a.shape[0]}x{b.shape[1]}x{a.shape[1]} beta{beta}", prog[0])
     return prog
 
@@ -153,7 +174,7 @@ def _program(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequen
 def cached_programs() -> list:
     """``(label, FusedProgram)`` of every lowered plan in the cache (for timeline tracing of programs that exist already)."""
     out = []
-    for key, (_ops, _layouts, prog) in _program_cache.items():
+    for key, (_ops, _form, prog) in list(_program_cache.items()):
         out.append((f"stationary_{key[0]} rank{key[4]} beta{key[6]}", prog[0]))
     return out
 
@@ -193,12 +214,13 @@ def _splits_k(a: DistMatrix, c: DistMatrix) -> bool:
 # ----------------------------------------------------------------------------- fused executor
 def _run_fused(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequence[MultiplyOp], *,
                fuse_replica_reduce: bool = True, barriers: bool = True, beta: int = 1,
-               checksum: torch.Tensor | None = None, gelu_out: DistMatrix | None = None) -> None:
+               checksum: torch.Tensor | None = None, gelu_out: DistMatrix | None = None, program=None) -> None:
+    """``program``: what :func:`_program` returned for this call, where the caller keeps it."""
     from ..ops.device import DeviceState
 
     world = c.world
     state = DeviceState.get(c.device)
-    prog, needs_zero = _program(kind, a, b, c, ops, fuse_replica_reduce, beta, gelu_out)
+    prog, needs_zero = program or _program(kind, a, b, c, ops, fuse_replica_reduce, beta, gelu_out)
     if needs_zero:        # several ranks add into C: clear it before the entry barrier lets anyone push
         pad = c.local_padded
         state.zero_2d(pad.data_ptr(), c.ld * c.itemsize, pad.shape[0], c.ld * c.itemsize)

@@ -150,7 +150,7 @@ class DistMatrix:
         """Release the symmetric allocation (collective: every rank frees the same matrix in the same order)."""
         from . import exec as _exec
 
-        _exec.drop_programs_for(self.buffer.ptr(self.rank))
+        _exec.drop_programs_for(self.buffer.uid)
         _registry.pop(self.buffer.ptr(self.rank), None)
         if self._dtensor is not None:
             _registry.pop(self._dtensor._local_tensor.data_ptr(), None)

@@ -34,16 +34,21 @@ class MatmulPlan:
             # executor (zero the non-origin replicas, reduce_replicas, barrier) is not part of a prepared plan.
             raise ValueError("a prepared plan of a replicated C needs fuse_replica_reduce=True "
                              "(use ug.matmul(..., fuse_replica_reduce=False) for the separate reduction pass)")
-        # lowering happens here; later calls hit the program cache by identity of the op list
+        # Lowering happens here.  The plan runs this program and no other: a graph holds the addresses of its tables, so
+        # they live as long as the plan, whatever becomes of the program cache.
         self.program, self.needs_zero = X._program(self.kind, self.a, self.b, self.c, self.ops, self.fuse, beta)
         self._graph: torch.cuda.CUDAGraph | None = None
+
+    def _launch(self) -> None:
+        X._run_fused(self.kind, self.a, self.b, self.c, self.ops, fuse_replica_reduce=self.fuse, beta=self.beta,
+                     program=(self.program, self.needs_zero))
 
     def run(self) -> None:
         """Queue one ``C (+)= A @ B`` on the current stream."""
         if self._graph is not None:
             self._graph.replay()
             return
-        X._run_fused(self.kind, self.a, self.b, self.c, self.ops, fuse_replica_reduce=self.fuse, beta=self.beta)
+        self._launch()
 
     __call__ = run
 
@@ -56,13 +61,13 @@ class MatmulPlan:
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):
             for _ in range(max(warmup, 1)):
-                X._run_fused(self.kind, self.a, self.b, self.c, self.ops, fuse_replica_reduce=self.fuse, beta=self.beta)
+                self._launch()
         torch.cuda.current_stream(dev).wait_stream(side)
         torch.cuda.synchronize(dev)
         self.c.world.barrier()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            X._run_fused(self.kind, self.a, self.b, self.c, self.ops, fuse_replica_reduce=self.fuse, beta=self.beta)
+            self._launch()
         self._graph = graph
         return self
 

@@ -18,6 +18,7 @@ reference (dtensor_scratch.py:9-53, dtensor_utils.py:30-115,546-552).
 from __future__ import annotations
 
 import ctypes
+import itertools
 import os
 import uuid
 import weakref
@@ -39,8 +40,14 @@ class GuardViolation(RuntimeError):
     """Something wrote outside a symmetric allocation (into one of its guard regions)."""
 
 
+_buffer_uids = itertools.count(1)
+
+
 class SymmBuffer:
     """One collective allocation as seen from one rank.
+
+    ``uid`` names this allocation in this process and is never given out again: addresses are (the allocator hands the
+    same ones out to later matrices, of other types and with other peers), so nothing is looked up by address alone.
 
     With ``guard`` > 0 the raw allocation is ``guard + nbytes + guard`` bytes: the payload sits between two regions
     filled with ``GUARD_BYTE`` that nothing may touch; ``check_guards`` looks at this rank's copy."""
@@ -48,6 +55,7 @@ class SymmBuffer:
     def __init__(self, world: "World", nbytes: int, ptrs: Sequence[int], tensors: Sequence[torch.Tensor | None],
                  closer=None, guard: int = 0):
         self.world = world
+        self.uid = next(_buffer_uids)
         self.guard = int(guard)
         self.nbytes = int(nbytes) - 2 * self.guard
         self._ptrs = [int(p) + self.guard for p in ptrs]
