@@ -855,3 +855,32 @@ def test_small_fp32_products_share_their_staged_copies(m, n, k, beta):
     want = full_a.double() @ full_b.double() + beta * full_c.double()
     assert (c.local.double() - want).norm() <= 3e-5 * want.norm()
     X.clear_program_cache()
+
+
+@pytest.mark.parametrize("tile_m", [128, 256, "pair"])
+def test_the_last_part_of_a_tile_sees_all_other_parts(tile_m):
+    """Every lane of the part that writes C reads what other SMs have just written: 100 launches over changing operands,
+    so that a sum of the launch before would show, each equal in every bit to a second launch on the same operands."""
+    from universal_gemm_b200.ops import native
+    from universal_gemm_b200.ops.gemm import run_program
+
+    m, n, k = 256, 1024, 2048
+    gen = torch.Generator(device=_dev()).manual_seed(9)
+    source = torch.randn(m, k, device=_dev(), generator=gen).bfloat16()
+    a = source.clone()
+    b = (torch.randn(k, n, device=_dev(), generator=gen) / k ** 0.5).bfloat16()
+    c = torch.zeros(m, n, device=_dev())
+    prog = _cut_program(a, b, c, native.C_STORE, tile_m, 8)
+    differ = torch.zeros((), dtype=torch.int64, device=_dev())
+    for i in range(50):
+        a.copy_(source.roll(i, 0))
+        run_program(prog, _dev())
+        first = c.clone()
+        if i == 0:
+            base = first
+        run_program(prog, _dev())
+        differ += (first != c).sum() + (first != base.roll(i, 0)).sum()
+    _status_ok()
+    assert int(differ) == 0
+    want = source.double() @ b.double()
+    assert (base.double() - want).norm() <= 1e-5 * want.norm()

@@ -533,11 +533,14 @@ __device__ __forceinline__ void part_done(uint32_t* counter, int lane) {
     red_add_gpu(counter, 1u);
   }
 }
-// Bounded wait of a whole warp for the other parts of a tile.
+// Bounded wait of a whole warp for the other parts of a tile.  Lane 0 acquires; the warp barrier orders the reads of the
+// other lanes after it (the shuffle alone orders no memory).
 __device__ __forceinline__ bool parts_wait(const uint32_t* counter, uint32_t need, int lane, const WaitCtl& ctl) {
   int ok = 1;
   if (lane == 0) ok = flag_wait(counter, need, ctl) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();
+  return ok != 0;
 }
 __device__ __forceinline__ bool part_in_bounds(const UgFusedParams& P, const UgTask& t) {
   return t.part_count <= 1 || (t.part_ptr != 0 && t.part_flag >= 0 && t.part_index >= 0 && t.part_index < t.part_count &&
