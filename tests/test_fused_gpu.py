@@ -884,3 +884,31 @@ def test_the_last_part_of_a_tile_sees_all_other_parts(tile_m):
     assert int(differ) == 0
     want = source.double() @ b.double()
     assert (base.double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 95, 97, 255, 279, 543])
+@pytest.mark.parametrize("tile_m", [128, 256, "pair"])
+def test_bf16_add_rounds_once_at_the_ragged_end(n, tile_m):
+    """bf16 ``C +=`` onto values that nearly cancel the product, in a C with aligned rows: the columns past the last whole
+    chunk of 32 add the fp32 sum and round once, so what is left is within half an ulp (2^-9 relative) of the exact value,
+    plus the error of the fp32 sum (k terms of order k^-1/2: 1e-6).  Rounding the product first would leave 2^-9 of the product."""
+    from universal_gemm_b200.ops import native
+    from universal_gemm_b200.ops.gemm import build_gemm_program, run_program
+
+    m, k = 200, 256
+    gen = torch.Generator(device=_dev()).manual_seed(10 + n)
+    a = torch.randn(m, k, device=_dev(), generator=gen).bfloat16()
+    b = torch.zeros(k, -(-n // 64) * 64, device=_dev(), dtype=torch.bfloat16)[:, :n]
+    b.copy_(torch.randn(k, n, device=_dev(), generator=gen) / k ** 0.5)
+    c = torch.zeros(m, -(-n // 64) * 64, device=_dev(), dtype=torch.bfloat16)[:, :n]
+    prod = a.double() @ b.double()
+    c.copy_(-prod)                                             # rounded to bf16: the sum is that rounding's error
+    want = prod + c.double()
+    run_program(build_gemm_program([a], [b], c, mode=native.C_ADD, tile_m=tile_m), _dev())
+    _status_ok()
+    # the two warps of a lane quadrant split a tile's columns at a multiple of 64, so chunks of 32 start at multiples of 32
+    ragged = n // 32 * 32
+    got, left = c[:, ragged:].double(), want[:, ragged:]
+    assert ((got - left).abs() <= 2.0 ** -9 * left.abs() + 2e-6).all()
+    whole, prod = (c.double() - want)[:, :ragged].abs(), prod[:, :ragged].abs()
+    assert (whole <= 2.0 ** -9 * prod + 2.0 ** -9 * want[:, :ragged].abs() + 2e-6).all()

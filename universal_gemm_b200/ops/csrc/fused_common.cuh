@@ -176,6 +176,10 @@ __device__ __forceinline__ bool task_c_pitch_vec(const UgTask& t) { return (t.c_
 // All rows share one 16-byte alignment phase (checked when the table is built).
 __device__ __forceinline__ bool task_c_rows_indirect(const UgTask& t) { return (t.c_vec & 4) != 0; }
 
+// Bit 3 of c_vec: a bf16 C that only this task adds to (c_mode 0) may take the reduction instruction where whole aligned
+// chunks are added; they round the sum to bf16 before they add it either way.  The ragged end of a row adds in fp32.
+__device__ __forceinline__ int task_chunk_mode(const UgTask& t) { return (t.c_vec & 8) != 0 ? 1 : t.c_mode; }
+
 // Where the 32 rows of an epilogue warp go: rows of one region (base + r * ldc) or rows named by a table.
 struct CRows {
   const uint64_t* tab;   // entry of the warp's first row, or nullptr
@@ -1012,7 +1016,7 @@ __device__ __forceinline__ void epilogue_drain(uint32_t taddr, const UgTask& t, 
       if (acc != nullptr && lane < rows_valid) *acc += sum_columns(v0, 0, 32) + sum_columns(v1, 0, 32);
       store_chunk_bf16_64(epi_buf, v0, v1, lane,
                           reinterpret_cast<__nv_bfloat16*>(t.c_ptr) + static_cast<int64_t>(row0) * t.ldc + col0 + c,
-                          t.ldc, rows_valid, t.c_mode);
+                          t.ldc, rows_valid, task_chunk_mode(t));
       c += 32;
       continue;
     }
@@ -1027,7 +1031,7 @@ __device__ __forceinline__ void epilogue_drain(uint32_t taddr, const UgTask& t, 
         store_chunk_f32(epi_buf, v, lane, reinterpret_cast<float*>(t.c_ptr) + off0, t.ldc, rows_valid, t.c_mode);
       else
         store_chunk_bf16(epi_buf, v, lane, reinterpret_cast<__nv_bfloat16*>(t.c_ptr) + off0, t.ldc, rows_valid,
-                         t.c_mode);
+                         task_chunk_mode(t));
     } else {
       store_chunk_scalar(epi_buf, v, lane, t.c_ptr, off0, t.ldc, rows_valid, ncols, t.c_mode, t.c_dtype);
     }

@@ -59,7 +59,9 @@ typedef struct __attribute__((aligned(16))) {
   int32_t kblocks;       // sum over segments of ceil(k_len / UG_BK)
   int32_t c_mode;        // 0: C += acc (plain read-modify-write), 1: red.add (atomic, any owner), 2: C = acc
   int32_t c_dtype;       // 0: fp32, 1: bf16
-  int32_t c_vec;         // 1 when 16-byte accesses to C rows are legal
+  int32_t c_vec;         // bit 0: 16-byte accesses to C rows are legal; bit 1: the row pitch is a multiple of 16 bytes; bit 2:
+                         // c_ptr is a table of row addresses; bit 3: whole chunks of a bf16 `C +=` may be reductions;
+                         // bits 16 and up: columns per tile (0: UG_BN)
   int32_t group_m;       // m tiles per raster band (L2 reuse of the A band)
   uint64_t act_ptr;      // 0, or where gelu(C) goes too, as bf16 with C's pitch (fp32 C that is stored, c_mode 2)
   // A tile whose K blocks are cut into part_count tasks (0: not cut).  Parts 0 .. part_count - 2 leave their fp32 sums at

@@ -525,16 +525,17 @@ class FusedProgramBuilder:
             if task.tile_n != BN:
                 c_vec |= task.tile_n << 16
             # C += acc by plain loads and stores waits for memory row by row (28 us for a tile of the 256-row variant,
-            # where nothing hides it); the reduction instruction does the same addition in bf16, subnormals included, and
-            # waits for nothing.  fp32 keeps the plain form: reductions into memory flush its subnormals.
-            mode = task.c_mode
-            if mode == native.C_ADD and task.c_dtype == native.DT_BF16 and c_vec & 1:
-                mode = native.C_ATOMIC
+            # where nothing hides it); in whole 32-column chunks of bf16, which round acc before they add it, the reduction
+            # instruction does the same addition, subnormals included, and waits for nothing.  The ragged end of a row
+            # keeps the plain form, which adds in fp32 and rounds once, and so does fp32: reductions into memory flush
+            # its subnormals.
+            if task.c_mode == native.C_ADD and task.c_dtype == native.DT_BF16 and c_vec & 1:
+                c_vec |= 8
             band = 2048 // BM
             group_m = m_tiles if m_tiles <= band else band
             task_rows.append(dict(c_ptr=task.c_ptr, ldc=task.ldc, m=task.m, n=task.n, seg_begin=seg_begin,
                                   seg_count=len(seg_rows) - seg_begin, tile_begin=tile_begin, m_tiles=m_tiles,
-                                  n_tiles=n_tiles, kblocks=kblocks, c_mode=mode, c_dtype=task.c_dtype,
+                                  n_tiles=n_tiles, kblocks=kblocks, c_mode=task.c_mode, c_dtype=task.c_dtype,
                                   c_vec=c_vec, group_m=group_m, act_ptr=task.act_ptr))
             if task.part[1] > 1:
                 index, count = task.part
