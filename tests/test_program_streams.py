@@ -1,0 +1,216 @@
+"""Launches of one program on several streams: they share its tables, staged copies, counters and workspace."""
+import threading
+
+import pytest
+import torch
+
+import universal_gemm_b200 as ug
+from universal_gemm_b200.ops import fused, native
+
+from helpers import make_inputs
+
+
+class _Cuda:
+    """The calls of torch.cuda that a program makes, written down."""
+
+    def __init__(self):
+        self.log, self.capturing, self.current = [], False, 0
+        outer = self
+
+        class Event:
+            def record(self, stream):
+                outer.log.append(("record", stream.raw))
+                self.at = len(outer.log)
+
+        class Stream:
+            def __init__(self, raw, device=None):
+                self.raw = self.cuda_stream = raw
+
+            def wait_event(self, event):
+                outer.log.append(("wait", self.raw, outer.log[event.at - 1][1]))
+
+        self.Event, self.ExternalStream = Event, Stream
+        self.default_stream = lambda device=None: Stream(0)
+        self.current_stream = lambda device=None: Stream(self.current)
+        self.is_current_stream_capturing = lambda: self.capturing
+
+
+class _Memory:
+    def __init__(self, log, name):
+        self.log, self.name = log, name
+
+    def record_stream(self, stream):
+        self.log.append(("used", self.name, stream.raw))
+
+
+@pytest.fixture
+def cuda(monkeypatch):
+    fake = _Cuda()
+    monkeypatch.setattr(torch, "cuda", fake)
+    return fake
+
+
+def _program(cuda, built_on=0):
+    cuda.current = built_on
+    params = native.FusedParams()
+    prog = fused.FusedProgram(device=torch.device("cuda", 0), tables=_Memory(cuda.log, "tables"), staging=None,
+                              workspace=_Memory(cuda.log, "workspace"), params=params, grid=148, clear_ptr=0, num_clear=0, stats={})
+    prog._entry = lambda ref, grid, stream: cuda.log.append(("launch", stream, params.checksum)) or 0
+
+    def launch(stream, checksum=0):
+        cuda.current = stream
+        prog.launch(stream, checksum)
+    return launch
+
+
+def test_the_default_stream_alone_costs_no_event(cuda):
+    launch = _program(cuda)
+    launch(0), launch(0, 7), launch(0)
+    assert cuda.log == [("launch", 0, 0), ("launch", 0, 7), ("launch", 0, 0)]
+
+
+def test_a_launch_on_another_stream_waits_for_the_last_and_keeps_the_memory(cuda):
+    launch = _program(cuda)
+    launch(0), launch(5), launch(5), launch(9), launch(0)
+    assert cuda.log == [("launch", 0, 0),
+                        ("record", 0), ("wait", 5, 0), ("used", "tables", 5), ("used", "workspace", 5), ("launch", 5, 0), ("record", 5),
+                        ("launch", 5, 0), ("record", 5),
+                        ("wait", 9, 5), ("used", "tables", 9), ("used", "workspace", 9), ("launch", 9, 0), ("record", 9),
+                        ("wait", 0, 9), ("used", "tables", 0), ("used", "workspace", 0), ("launch", 0, 0)]
+
+
+def test_the_first_launch_waits_for_the_stream_that_built_the_tables(cuda):
+    launch = _program(cuda, built_on=3)
+    launch(0)
+    assert cuda.log == [("record", 3), ("wait", 0, 3), ("used", "tables", 0), ("used", "workspace", 0), ("launch", 0, 0)]
+
+
+def test_a_captured_launch_leaves_events_alone(cuda):
+    """A captured stream must not wait for an event from outside, nor leave one behind."""
+    launch = _program(cuda)
+    cuda.capturing = True
+    launch(5)
+    cuda.capturing = False
+    launch(0)
+    assert cuda.log == [("launch", 5, 0), ("launch", 0, 0)]
+
+
+def test_every_thread_s_launch_has_its_own_checksum(cuda):
+    launch = _program(cuda)
+    threads = [threading.Thread(target=lambda i=i: [launch(0, i) for _ in range(200)]) for i in range(1, 5)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert sorted(x[2] for x in cuda.log) == sorted([1, 2, 3, 4] * 200)
+
+
+def _dev():
+    return torch.device("cuda", torch.cuda.current_device())
+
+
+def _zero_counters(prog):
+    """Every word that a launch expects to be zero."""
+    torch.cuda.synchronize()
+    p, base = prog.params, prog._tables.data_ptr()
+    words = [(p.flags, p.num_flags + 2 if p.num_pieces else 0), (p.part_flags, p.num_part_flags), (p.sched, 1 if p.sched else 0),
+             (p.finished, 1 if p.finished else 0)]
+    return all(int(prog._tables[at - base:at - base + 4 * n].view(torch.int32).abs().sum()) == 0 for at, n in words if n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile_m", [128, 256, "pair"])
+@pytest.mark.parametrize("staged", [False, True])
+def test_launches_on_changing_streams(tile_m, staged):
+    """Cut tiles and staged operands, launched in turn on three streams that nothing else orders: C += adds up."""
+    from universal_gemm_b200.ops.device import DeviceState, torch_dtype_code
+    from universal_gemm_b200.ops.gemm import _segments, _slice_of, run_program
+
+    m, n, k = 300, 1030, 2304
+    gen = torch.Generator(device=_dev()).manual_seed(3)
+    a = torch.randn(m, k, device=_dev(), generator=gen).bfloat16()
+    b = torch.zeros(k, 1088, device=_dev(), dtype=torch.bfloat16)[:, :n]
+    b.copy_(torch.randn(k, n, device=_dev(), generator=gen) / k ** 0.5)
+    c = torch.zeros(m, n, device=_dev())
+    st = DeviceState.get(_dev())
+    builder = fused.FusedProgramBuilder(_dev(), num_sms=st.num_sms, tile_m=tile_m, parts=3)
+    builder.add_task(fused.TaskSpec(c_ptr=c.data_ptr(), ldc=n, m=m, n=n, c_mode=native.C_ADD, c_dtype=torch_dtype_code(c.dtype),
+                                    segments=_segments(_slice_of(a, remote=staged), _slice_of(b, remote=staged))))
+    prog = builder.build(st.status_ptr)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.current_stream()]
+    torch.cuda.synchronize()
+    for i in range(30):
+        with torch.cuda.stream(streams[i % 3]):
+            run_program(prog, _dev())
+    assert _zero_counters(prog)
+    ug.check_status(_dev())
+    want = 30 * (a.double() @ b.double())
+    assert (c.double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.gpu
+def test_a_program_dropped_while_another_stream_runs_it():
+    """Its tables and staging area go back to the allocator only when that stream is done with them."""
+    from universal_gemm_b200.parallel import exec as X
+
+    m, n, k = 515, 700, 4100
+    full_a, full_b, _ = make_inputs(m, n, k, seed=44, device=_dev())
+    world = ug.EmulatedCluster(2, _dev()).worlds()
+    mats = [(ug.distribute_tensor(full_a, w, "block", dtype=torch.bfloat16), ug.distribute_tensor(full_b, w, "row", dtype=torch.bfloat16),
+             ug.zeros(w, (m, n), "column", torch.float32)) for w in world]
+    side = torch.cuda.Stream()
+    X.clear_program_cache()
+    for a, b, c in mats:
+        ug.matmul(a, b, c, method="stationary_c", beta=0)
+    torch.cuda.synchronize()
+    sizes = [(p._tables.numel(), p._staging.numel()) for _, p in X.cached_programs()]
+    for _ in range(20):
+        for a, b, c in mats:
+            c.local_padded.zero_()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                for a, b, c in mats:
+                    ug.matmul(a, b, c, method="stationary_c", beta=0)
+        X.clear_program_cache()
+        for pair in sizes:                       # would get the memory of a program that still runs
+            for size in pair:
+                torch.full((size,), 0xFF, dtype=torch.uint8, device=_dev())
+        torch.cuda.current_stream().wait_stream(side)
+        for a, b, c in mats:                     # lowered again, on the default stream
+            ug.matmul(a, b, c, method="stationary_c", beta=0)
+    torch.cuda.synchronize()
+    ug.check_status(_dev())
+    want = full_a.bfloat16().double() @ full_b.bfloat16().double()
+    torch.testing.assert_close(mats[0][2].full_tensor().double(), want, rtol=2e-3, atol=2e-3)
+    X.clear_program_cache()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tile_m", [(torch.bfloat16, "pair"), (torch.bfloat16, "128"), (torch.float32, "pair"), (torch.float32, "128")])
+def test_counters_are_back_at_zero_after_replays(dtype, tile_m, monkeypatch):
+    """Chunk counters, piece cursor, tile claim and finished workers of claimed (pair) and staged (fp32) programs, replayed
+    from a graph on two streams that only the program orders, with an eager call between."""
+    from universal_gemm_b200.parallel import exec as X
+
+    monkeypatch.setenv("UGEMM_TILE_M", tile_m)
+    m, n, k = 515, 2100, 2100
+    full_a, full_b, _ = make_inputs(m, n, k, seed=43, device=_dev())
+    world = ug.SingleWorld(_dev())
+    a, b = ug.distribute_tensor(full_a, world, "row", dtype=dtype), ug.distribute_tensor(full_b, world, "column", dtype=dtype)
+    c = ug.zeros(world, (m, n), "row", torch.float32)
+    plan = ug.prepare_matmul(a, b, c, beta=0).capture()
+    assert plan.program.params.finished != 0 or plan.program.params.sched == 0
+    side = torch.cuda.Stream()
+    for i in range(6):
+        c.local_padded.fill_(9.0)
+        torch.cuda.synchronize()
+        plan()
+        with torch.cuda.stream(side):
+            plan()
+        ug.matmul(a, b, c, beta=0)
+        assert _zero_counters(plan.program)
+    ug.check_status(_dev())
+    want = full_a.to(dtype).double() @ full_b.to(dtype).double()
+    assert (c.local.double() - want).norm() <= 3e-5 * want.norm()
+    X.clear_program_cache()

@@ -893,12 +893,13 @@ __device__ __forceinline__ void trace_fetch(const UgFusedParams& P, int cta, int
 
 // Called by all threads of a worker's CTA (the leader's, of a pair) once every role of the worker is done: the last
 // worker of the launch puts the counters back to zero, so that the next launch needs no clearing pass before it
-// (2.3 us and a launch gap per call).
+// (2.3 us and a launch gap per call).  The count of finished workers wraps by itself: should two launches of a program
+// overlap after all (replays of one graph on two streams), it and with it every counter is back at zero when both are done.
 __device__ __forceinline__ void rearm_counters(const UgFusedParams& P, uint32_t workers, uint32_t* last) {
   if (P.finished == 0) return;
   if (threadIdx.x == 0) {
     __threadfence();
-    *last = atomicAdd(reinterpret_cast<uint32_t*>(P.finished), 1u) == workers - 1u ? 1u : 0u;
+    *last = atomicInc(reinterpret_cast<uint32_t*>(P.finished), workers - 1u) == workers - 1u ? 1u : 0u;
     __threadfence();
   }
   __syncthreads();
@@ -908,10 +909,7 @@ __device__ __forceinline__ void rearm_counters(const UgFusedParams& P, uint32_t 
     for (int i = threadIdx.x; i < P.num_flags + 2; i += blockDim.x) flags[i] = 0u;
   uint32_t* part_flags = reinterpret_cast<uint32_t*>(P.part_flags);
   for (int i = threadIdx.x; i < P.num_part_flags; i += blockDim.x) part_flags[i] = 0u;
-  if (threadIdx.x == 0) {
-    if (P.sched != 0) *reinterpret_cast<uint32_t*>(P.sched) = 0u;
-    *reinterpret_cast<uint32_t*>(P.finished) = 0u;
-  }
+  if (threadIdx.x == 0 && P.sched != 0) *reinterpret_cast<uint32_t*>(P.sched) = 0u;
 }
 
 // Store a 32 x 32 block of fp32 C and, as bf16, its gelu (an MLP's hidden layer: the activation is the operand of the

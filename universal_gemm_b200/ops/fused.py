@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from bisect import bisect_left, bisect_right
 from dataclasses import dataclass, field, replace
 from typing import Callable, Sequence
@@ -191,8 +192,17 @@ class _Staged:
     low: "_Staged | None" = None         # high part of a split fp32 slice: where the low part goes
 
 
+def _stream(raw: int, device: torch.device):
+    return torch.cuda.ExternalStream(raw, device=device) if raw else torch.cuda.default_stream(device)
+
+
 class FusedProgram:
-    """Device-resident tables of one lowered plan, ready to launch."""
+    """Device-resident tables of one lowered plan, ready to launch.
+
+    Launches of one program share its tables, staged copies, counters and workspace, so they run one after the other: a
+    launch on another stream than the last one waits for that one, and the memory is marked as used on every stream that
+    launches it (it belongs to the stream it was built on, which would get it back while another still runs).  Replays of
+    a graph that a caller captured cannot be seen from here: whoever replays it orders them."""
 
     def __init__(self, *, device: torch.device, tables: torch.Tensor, staging: torch.Tensor | None,
                  workspace: torch.Tensor | None, params: native.FusedParams, grid: int, clear_ptr: int, num_clear: int, stats: dict):
@@ -208,6 +218,11 @@ class FusedProgram:
         self._trace: torch.Tensor | None = None
         self._entry = native.lib().ug_fused_gemm_pair if params.cta_pair else native.lib().ug_fused_gemm
         self._params_ref = ctypes.byref(params)
+        self._lock = threading.Lock()
+        self._last = torch.cuda.current_stream(device).cuda_stream if device.type == "cuda" else 0    # stream of the last launch
+        self._done = None                      # event after it, unless that was the default stream, which is always there to ask
+        if self._last:
+            self._mark()
 
     # ------------------------------------------------------------------ optional per-tile timeline
     def enable_trace(self, slots: int | None = None) -> None:
@@ -248,8 +263,44 @@ class FusedProgram:
             native.check(native.lib().ug_zero_2d(self.clear_ptr, self.num_clear * 4, 1, self.num_clear * 4,
                                                  ctypes.c_void_p(stream)), "ug_zero_2d(flags)")
 
-    def launch(self, stream: int) -> None:
+    def launch(self, stream: int, checksum: int = 0) -> None:
+        """Queue one launch on ``stream`` (the current stream); ``checksum``: address of the double it adds its sum to."""
+        self.run_on(stream, self._call, stream, checksum)
+
+    def _call(self, stream: int, checksum: int) -> None:
+        self.params.checksum = checksum
         native.check(self._entry(self._params_ref, self.grid, stream), "ug_fused_gemm")
+
+    def run_on(self, stream: int, queue: Callable, *args) -> None:
+        """``queue(*args)`` puts a launch of this program (or the replay of a graph with one) on ``stream``, the current one."""
+        with self._lock:
+            if stream != self._last:
+                self._change_stream(stream)
+            queue(*args)
+            if stream:
+                self._mark()
+
+    def _mark(self) -> None:
+        if torch.cuda.is_current_stream_capturing():
+            return
+        if self._done is None:
+            self._done = torch.cuda.Event()
+        self._done.record(torch.cuda.current_stream(self.device))
+
+    def _change_stream(self, stream: int) -> None:
+        if torch.cuda.is_current_stream_capturing():
+            return
+        after = self._done
+        if not self._last:
+            after = torch.cuda.Event()
+            after.record(_stream(0, self.device))
+        new = _stream(stream, self.device)
+        if after is not None:
+            new.wait_event(after)
+        for t in (self._tables, self._staging, self._workspace):
+            if t is not None:
+                t.record_stream(new)
+        self._last = stream
 
 
 def _k_edges(k: int) -> tuple[int, ...]:

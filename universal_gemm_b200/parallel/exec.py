@@ -240,11 +240,7 @@ def _run_fused(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequ
     if checksum is not None:
         if checksum.dtype != torch.float64 or checksum.numel() < 1 or checksum.device != c.device:
             raise ValueError("checksum must be a float64 tensor on the device of C")
-        prog.params.checksum = checksum.data_ptr()
-    try:
-        prog.launch(state.stream())
-    finally:
-        prog.params.checksum = 0
+    prog.launch(state.stream(), checksum.data_ptr() if checksum is not None else 0)
     state.launches += 1
     if prof:
         e2.record()

@@ -13,6 +13,7 @@ from typing import Any
 
 import torch
 
+from ..ops.device import DeviceState
 from . import exec as X
 from . import plan as P
 from .matrix import resolve
@@ -46,7 +47,7 @@ class MatmulPlan:
     def run(self) -> None:
         """Queue one ``C (+)= A @ B`` on the current stream."""
         if self._graph is not None:
-            self._graph.replay()
+            self.program.run_on(DeviceState.get(self.c.device).stream(), self._graph.replay)
             return
         self._launch()
 
