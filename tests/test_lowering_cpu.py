@@ -208,3 +208,21 @@ def test_k_spans_of_a_split_product_put_the_small_terms_first():
         + [(1, 1, 0, 2200)]
     cut = FusedProgramBuilder._spans(segs, (7, 100))
     assert sum((n + 63) // 64 for *_, n in cut) == 93 and cut[0][2:] == (192, 64)
+
+
+def test_static_tiles_are_not_cut(monkeypatch):
+    """UGEMM_DYNAMIC_TILES=0 deals tiles round-robin; the parts of a cut tile need claims, so there are none then, and the
+    time model counts the last wave as it runs."""
+    def builder(**kw):
+        b = FusedProgramBuilder("cpu", num_sms=148, **kw)
+        b.add_task(_task(64, 16384, 16384))              # 64 tiles, 256 K blocks each
+        return b
+
+    assert builder()._choose_parts(builder().tasks, 128)[1] > 1
+    cut_us = builder().model_us(128)
+    monkeypatch.setenv("UGEMM_DYNAMIC_TILES", "0")
+    assert builder()._choose_parts(builder().tasks, 128)[1] == 1
+    assert builder().model_us(128) > cut_us
+    assert builder(parts=4)._choose_parts(builder().tasks, 128) is None
+    monkeypatch.setenv("UGEMM_DYNAMIC_TILES", "1")
+    assert builder()._choose_parts(builder().tasks, 128)[1] > 1

@@ -885,8 +885,9 @@ class FusedProgramBuilder:
         bm = v["rows"]
         counts = [((t.m + bm - 1) // bm) * ((t.n + BN - 1) // BN) for t in tasks]
         total = sum(counts)
+        claimed = os.environ.get("UGEMM_DYNAMIC_TILES", "") != "0"       # without claims a part might wait for a part behind it
         if self.parts is not None:
-            return (total, self.parts, 0.0) if min(t.total_blocks() for t in tasks) >= self.parts else None
+            return (total, self.parts, 0.0) if claimed and min(t.total_blocks() for t in tasks) >= self.parts else None
         blocks = {t.total_blocks() for t in tasks}
         tail = total % workers
         if len(blocks) != 1 or tail == 0 or any(t.tile_n != BN for t in tasks):
@@ -901,7 +902,7 @@ class FusedProgramBuilder:
         plain = whole
         if total > workers and 2 * tail <= workers and self._split_tail(tasks, bm, workers) != tasks:
             plain = (total // workers + 0.7) * tile
-        taken = self._tail_tiles(tasks, bm, tail)
+        taken = self._tail_tiles(tasks, bm, tail) if claimed else None
         if taken is None:
             return 0, 1, whole - plain
         _, tail = taken
