@@ -226,3 +226,17 @@ def test_static_tiles_are_not_cut(monkeypatch):
     assert builder(parts=4)._choose_parts(builder().tasks, 128) is None
     monkeypatch.setenv("UGEMM_DYNAMIC_TILES", "1")
     assert builder()._choose_parts(builder().tasks, 128)[1] > 1
+
+
+def test_the_time_model_is_evaluated_once_per_variant(monkeypatch):
+    calls = []
+    evaluate = FusedProgramBuilder._evaluate
+    monkeypatch.setattr(FusedProgramBuilder, "_evaluate", lambda self, variant: calls.append(variant) or evaluate(self, variant))
+    b = FusedProgramBuilder("cpu", num_sms=148)
+    b.add_task(_task(64, 16384, 16384))
+    variant = b.choose_tile_m()
+    first = b.model_us(variant)
+    b.choose_tile_m()
+    assert len(calls) == 3 and len(set(calls)) == 3
+    b.add_task(_task(64, 16384, 16384))                  # other tasks, another answer
+    assert b.model_us(variant) > first and len(calls) == 4

@@ -332,6 +332,7 @@ class FusedProgramBuilder:
             raise ValueError('tile_m must be 128, 256, "pair" or "pair512"')
         self.tile_m = tile_m
         self.tasks: list[TaskSpec] = []
+        self._models: dict = {}      # variant -> (microseconds, cut) of the tasks so far
 
     def merge_row_tasks(self, max_rows: int = 256) -> int:
         """Merge tasks that multiply different rows of A with the same B slices (and write equally wide regions of an
@@ -371,6 +372,7 @@ class FusedProgramBuilder:
                                        tile_n=take[0].tile_n, c_rows=tuple((t.c_ptr, t.ldc, t.m) for t in take)))
         saved = len(self.tasks) - len(merged)
         self.tasks = merged
+        self._models.clear()
         return saved
 
     def add_task(self, task: TaskSpec) -> None:
@@ -381,6 +383,7 @@ class FusedProgramBuilder:
                 raise ValueError(f"inconsistent segment shapes: A {a.rows}x{a.cols}, B {b.rows}x{b.cols}, "
                                  f"C {task.m}x{task.n}")
         self.tasks.append(task)
+        self._models.clear()
 
     # ------------------------------------------------------------------ tile shape
     def choose_tile_m(self):
@@ -404,10 +407,19 @@ class FusedProgramBuilder:
     def model_us(self, variant) -> float | None:
         """Modelled kernel time in microseconds of the tasks added so far under tile variant ``variant`` (the busiest
         worker of the model described in :meth:`choose_tile_m`); ``None`` when the variant cannot run here."""
+        return self._model(variant)[0]
+
+    def _model(self, variant) -> tuple[float | None, tuple[int, int, float] | None]:
+        """``(model_us, what _choose_parts says)``, worked out once per variant: lowering asks for them several times."""
+        if variant not in self._models:
+            self._models[variant] = self._evaluate(variant)
+        return self._models[variant]
+
+    def _evaluate(self, variant) -> tuple[float | None, tuple[int, int, float] | None]:
         v = _VARIANTS[variant]
         workers = self.num_sms // 2 if v["pair"] else self.num_sms
         if workers < 1:
-            return None
+            return None, None
         per_worker = [0.0] * workers
         tile = 0
         last = 0.0
@@ -429,8 +441,8 @@ class FusedProgramBuilder:
             for _ in range(rest):
                 per_worker[tile % workers] += cost
                 tile += 1
-        cut = self._choose_parts(tasks, variant) if self.parts is None else None
-        return max(per_worker) + last - (cut[2] if cut is not None else 0.0)
+        cut = self._choose_parts(tasks, variant)
+        return max(per_worker) + last - (cut[2] if cut is not None else 0.0), cut
 
     @staticmethod
     def _epilogue_us(t: TaskSpec, v: dict) -> float:
@@ -455,7 +467,7 @@ class FusedProgramBuilder:
         tasks = self.tasks
         if wide:
             tasks = [replace(t, tile_n=2 * BN) if t.tile_n == BN else t for t in tasks]
-        cut = self._choose_parts(tasks, variant)
+        modelled_us, cut = self._model(variant)
         if cut is not None and cut[1] > 1:
             tasks = self._cut_parts(tasks, BM, cut[0], cut[1])
         elif os.environ.get("UGEMM_TAIL_SPLIT", "1") != "0":
@@ -784,8 +796,7 @@ class FusedProgramBuilder:
         # capacity, and loads over NVLink hold it three times as long); eight still copy at 435 GB/s and cost 10 %.
         # A plan that needs its remote bytes no faster than 300 GB/s over its modelled kernel time takes eight.
         remote_total = sum(st.src.remote_bytes() for st in staged.values() if st.pieces_of is None)
-        modelled_us = self.model_us(variant) or 0.0
-        need_gbs = remote_total / (modelled_us * 1e3) if modelled_us > 0 else float("inf")
+        need_gbs = remote_total / (modelled_us * 1e3) if modelled_us else float("inf")
         params.fetch_depth = int(os.environ.get("UGEMM_FETCH_DEPTH", "0")) or (8 if need_gbs < 300.0 else 16)
         params.fetch_helpers = 1
         params.timeout_ns = self.timeout_ns
@@ -794,7 +805,7 @@ class FusedProgramBuilder:
                      indirect_rows=len(row_table), cut_tiles=num_part_flags // 16,
                      parts=cut[1] if cut is not None else 1, fetch_depth=int(params.fetch_depth),
                      push_bytes=sum(t.m * t.n * (4 if t.c_dtype == native.DT_F32 else 2) for t in tasks if t.c_remote),
-                     model_us=round(self.model_us(variant) or 0.0, 1),
+                     model_us=round(modelled_us or 0.0, 1),
                      remote_bytes=sum(st.src.remote_bytes() for st in staged.values() if st.pieces_of is None),
                      grid=grid)
         return FusedProgram(device=dev, tables=tables, staging=staging, workspace=workspace, params=params, grid=grid,
