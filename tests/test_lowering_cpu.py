@@ -240,3 +240,19 @@ def test_the_time_model_is_evaluated_once_per_variant(monkeypatch):
     assert len(calls) == 3 and len(set(calls)) == 3
     b.add_task(_task(64, 16384, 16384))                  # other tasks, another answer
     assert b.model_us(variant) > first and len(calls) == 4
+
+
+def test_workspaces_of_all_programs_are_bounded(monkeypatch):
+    """With the device's share used up, a program runs its last wave whole; an explicit number of parts stands."""
+    from universal_gemm_b200.ops import fused
+
+    def parts(**kw):
+        b = FusedProgramBuilder("cpu", num_sms=148, **kw)
+        b.add_task(_task(64, 16384, 16384))              # 64 tiles of 128 x 256: one other part's sums are 8 MiB
+        return b._choose_parts(b.tasks, 128)[1]
+
+    assert parts() == 2
+    monkeypatch.setitem(fused._workspace_bytes, None, fused._MAX_WORKSPACE_BYTES - (8 << 20))
+    assert parts() == 2
+    monkeypatch.setitem(fused._workspace_bytes, None, fused._MAX_WORKSPACE_BYTES - (8 << 20) + 1)
+    assert parts() == 1 and parts(parts=4) == 4

@@ -214,3 +214,20 @@ def test_counters_are_back_at_zero_after_replays(dtype, tile_m, monkeypatch):
     want = full_a.to(dtype).double() @ full_b.to(dtype).double()
     assert (c.local.double() - want).norm() <= 3e-5 * want.norm()
     X.clear_program_cache()
+
+
+@pytest.mark.gpu
+def test_a_program_s_workspace_is_accounted_for_while_it_lives():
+    from universal_gemm_b200.ops.device import DeviceState
+    from universal_gemm_b200.ops.gemm import _segments, _slice_of
+
+    st = DeviceState.get(_dev())
+    a, b, c = (torch.zeros(256, 256, device=_dev(), dtype=d) for d in (torch.bfloat16, torch.bfloat16, torch.float32))
+    before = fused._workspace_bytes.get(st.device.index, 0)
+    builder = fused.FusedProgramBuilder(st.device, num_sms=st.num_sms, tile_m=128, parts=3)
+    builder.add_task(fused.TaskSpec(c_ptr=c.data_ptr(), ldc=256, m=256, n=256, c_mode=native.C_STORE, c_dtype=native.DT_F32,
+                                    segments=_segments(_slice_of(a), _slice_of(b))))
+    prog = builder.build(st.status_ptr)
+    assert fused._workspace_bytes[st.device.index] - before == prog._workspace.numel() * 4 >= 2 * 2 * 128 * 256 * 4
+    del prog
+    assert fused._workspace_bytes[st.device.index] == before

@@ -18,6 +18,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import weakref
 from bisect import bisect_left, bisect_right
 from dataclasses import dataclass, field, replace
 from typing import Callable, Sequence
@@ -43,6 +44,8 @@ _VARIANTS = {
 _CUT_US = 5.0                            # what cutting costs whatever the parts: the first claim, writing the sums, waiting for them
 _MAX_PARTS = 8                           # K parts of a tile: each one more is another pass of the last part over the tile
 _MAX_PART_BYTES = 128 << 20              # workspace of one program
+_MAX_WORKSPACE_BYTES = 1 << 30           # workspaces of all programs of a device: with it used up, later programs cut no tiles
+_workspace_bytes: dict[int | None, int] = {}      # device index -> workspaces of the programs that are alive
 _AUTO_VARIANTS = (128, 256, "pair")      # "pair512" measured level with 256 and quantises worse: on request only
 _REMOTE_EPILOGUE_FACTOR = 1.3            # epilogue into a peer's C against local stores (10.6-11.1 vs 9.2 us on 2 GPUs)
 
@@ -311,6 +314,10 @@ def _k_edges(k: int) -> tuple[int, ...]:
         edges.append(at)
         at += min(at, 1024)
     return tuple(edges + [k])
+
+
+def _give_back_workspace(index: int | None, nbytes: int) -> None:
+    _workspace_bytes[index] -= nbytes
 
 
 class FusedProgramBuilder:
@@ -808,9 +815,14 @@ class FusedProgramBuilder:
                      model_us=round(modelled_us or 0.0, 1),
                      remote_bytes=sum(st.src.remote_bytes() for st in staged.values() if st.pieces_of is None),
                      grid=grid)
-        return FusedProgram(device=dev, tables=tables, staging=staging, workspace=workspace, params=params, grid=grid,
+        prog = FusedProgram(device=dev, tables=tables, staging=staging, workspace=workspace, params=params, grid=grid,
                             clear_ptr=0, num_clear=0,      # the kernel puts its counters back to zero itself
                             stats=stats)
+        if workspace is not None:
+            nbytes = workspace.numel() * 4
+            _workspace_bytes[dev.index] = _workspace_bytes.get(dev.index, 0) + nbytes
+            weakref.finalize(prog, _give_back_workspace, dev.index, nbytes).atexit = False
+        return prog
 
     @staticmethod
     def _spans(segments, k_blocks=None):
@@ -920,8 +932,9 @@ class FusedProgramBuilder:
         full, rest = divmod(total - tail, workers)
         part_us = v["part_us"] * min(1.0, max(t.m for t in tasks) / bm)     # only rows that exist are read
         best = None
+        room = min(_MAX_PART_BYTES, _MAX_WORKSPACE_BYTES - _workspace_bytes.get(self.device.index, 0))
         for p in range(2, _MAX_PARTS + 1):
-            if kb // p < 4 or tail * (p - 1) * bm * BN * 4 > _MAX_PART_BYTES:
+            if kb // p < 4 or tail * (p - 1) * bm * BN * 4 > room:
                 break
             part = self._tile_us(-(-kb // p), epi, v)
             # greedy: `workers - rest` workers are free after `full` tiles, `rest` one tile later
