@@ -101,7 +101,6 @@ def main() -> None:
         prog = builder.build(st.status_ptr)
 
         def fused(prog=prog):
-            prog.reset_flags(st.stream())
             prog.launch(st.stream())
 
         ms = timed(world, fused, args.iters)
@@ -115,7 +114,6 @@ def main() -> None:
         prog2 = builder.build(st.status_ptr)
 
         def fused_wide(prog2=prog2):
-            prog2.reset_flags(st.stream())
             prog2.launch(st.stream())
 
         ms = timed(world, fused_wide, args.iters)

@@ -209,7 +209,7 @@ def test_bounded_wait_reports_timeout_instead_of_hanging():
     slots = torch.zeros(2, 8, dtype=torch.int32, device=_dev())      # "rank 1" never adds to our slot
     table = torch.tensor([slots[0].data_ptr(), slots[1].data_ptr()], dtype=torch.int64, device=_dev())
     rounds = torch.zeros(1, dtype=torch.int32, device=_dev())
-    native.check(native.lib().ug_signal_barrier(table.data_ptr(), 2, 0, rounds.data_ptr(), st.status_ptr, 50_000_000, 0, 0,
+    native.check(native.lib().ug_signal_barrier(table.data_ptr(), 2, 0, rounds.data_ptr(), st.status_ptr, 50_000_000,
                                                 ctypes.c_void_p(st.stream())), "ug_signal_barrier")
     torch.cuda.synchronize()
     with pytest.raises(KernelStatusError) as err:
@@ -414,7 +414,6 @@ def test_beta_zero_with_separate_replica_reduction_clears_every_replica():
     for _, _, c in mats:                 # what every rank's executor does before its entry barrier
         c.local_padded.zero_()
     for prog in progs:                   # the ranks' kernels, one after the other
-        prog.reset_flags(st.stream())
         prog.launch(st.stream())
     for _, _, c in mats:
         R.reduce_replicas(c)
@@ -522,7 +521,6 @@ def test_skinny_problem_splits_k_across_the_gpu(method, triple):
     for _, c in progs:
         c.local_padded.zero_()
     for prog, _ in progs:
-        prog.reset_flags(st.stream())
         prog.launch(st.stream())
     _status_ok()
     torch.testing.assert_close(mats[0][2].full_tensor().double(), prod, rtol=2e-3, atol=2e-3)
@@ -718,7 +716,7 @@ def test_matmul_gelu_on_several_ranks(method, triple):
 
 
 def test_counters_are_back_at_zero_after_a_launch():
-    """Programs that stage operands run many times without a clearing pass, under capture too."""
+    """Programs that stage operands run many times without a clearing pass."""
     from universal_gemm_b200.parallel import exec as X
 
     m, n, k = 515, 700, 2100
@@ -733,10 +731,14 @@ def test_counters_are_back_at_zero_after_a_launch():
             c.local_padded.fill_(9.0)
             ug.matmul(a, b, c, method="stationary_c", beta=0)
     for label, prog in X.cached_programs():
-        assert prog.params.num_pieces > 0 and prog.num_clear == 0
+        assert prog.params.num_pieces > 0 and prog.params.finished != 0
         at = prog.params.flags - prog._tables.data_ptr()
         words = prog._tables[at:at + 4 * (prog.params.num_flags + 2)].view(torch.int32)
         assert int(words.abs().sum()) == 0, label
+        for at in (prog.params.sched, prog.params.finished):          # the next claim of a tile, the workers that are done
+            if at:
+                at -= prog._tables.data_ptr()
+                assert int(prog._tables[at:at + 4].view(torch.int32)) == 0, label
     _status_ok()
     torch.testing.assert_close(mats[0][2].full_tensor().double(), want, rtol=2e-3, atol=2e-3)
     X.clear_program_cache()

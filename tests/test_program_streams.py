@@ -54,7 +54,7 @@ def _program(cuda, built_on=0):
     cuda.current = built_on
     params = native.FusedParams()
     prog = fused.FusedProgram(device=torch.device("cuda", 0), tables=_Memory(cuda.log, "tables"), staging=None,
-                              workspace=_Memory(cuda.log, "workspace"), params=params, grid=148, clear_ptr=0, num_clear=0, stats={})
+                              workspace=_Memory(cuda.log, "workspace"), params=params, grid=148, stats={})
     prog._entry = lambda ref, grid, stream: cuda.log.append(("launch", stream, params.checksum)) or 0
 
     def launch(stream, checksum=0):
@@ -231,3 +231,35 @@ def test_a_program_s_workspace_is_accounted_for_while_it_lives():
     assert fused._workspace_bytes[st.device.index] - before == prog._workspace.numel() * 4 >= 2 * 2 * 128 * 256 * 4
     del prog
     assert fused._workspace_bytes[st.device.index] == before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile_m", [128, 256, "pair"])
+def test_counters_are_back_at_zero_after_a_launch_that_gave_up(tile_m):
+    """A chunk counter that never gets there (one piece more than there are) runs into the launch's limit and reports a
+    status; the launch after it starts from zero and is correct."""
+    from universal_gemm_b200.ops.device import DeviceState, KernelStatusError
+    from universal_gemm_b200.ops.gemm import build_gemm_program, run_program
+
+    st = DeviceState.get(_dev())
+    m, n, k = 300, 520, 700
+    gen = torch.Generator(device=_dev()).manual_seed(12)
+    a = torch.randn(m, k, device=_dev(), generator=gen).bfloat16()
+    b = (torch.randn(k, n, device=_dev(), generator=gen) / k ** 0.5).bfloat16()
+    c = torch.zeros(m, n, device=_dev())
+    prog = build_gemm_program([a], [b], c, mode=native.C_STORE, tile_m=tile_m, stage_a=True, stage_b=True, timeout_ns=200_000_000)
+    at = prog.params.flag_need - prog._tables.data_ptr()
+    need = prog._tables[at:at + 4 * prog.params.num_flags].view(torch.int32)
+    need += 1
+    run_program(prog, _dev())
+    torch.cuda.synchronize()
+    with pytest.raises(KernelStatusError) as err:
+        st.check()
+    assert err.value.code in (native.ERR_TIMEOUT_FLAG, native.ERR_TIMEOUT_MBAR)
+    assert _zero_counters(prog)
+    need -= 1
+    run_program(prog, _dev())
+    ug.check_status(_dev())
+    assert _zero_counters(prog)
+    want = a.double() @ b.double()
+    assert (c.double() - want).norm() <= 1e-5 * want.norm()

@@ -25,16 +25,13 @@ constexpr int kBarrierThreads = 256;
 
 __global__ void __launch_bounds__(kBarrierThreads) signal_barrier_kernel(
     const uint64_t* __restrict__ peer_slots, int world, int rank, uint32_t* seq_counter, uint32_t* status,
-    uint64_t timeout_ns, uint32_t* clear_ptr, int num_clear) {
+    uint64_t timeout_ns) {
   // The barrier's sequence number lives in device memory and advances by one per launch, so a captured
   // launch can be replayed (a CUDA graph of barrier + GEMM + barrier) and still wait for the right round.
   __shared__ uint32_t s_seq;
   if (threadIdx.x == 0) s_seq = atomicAdd(seq_counter, 1u) + 1u;
   __syncthreads();
   const uint32_t seq = s_seq;
-  // Plan-local words (chunk counters, piece cursor) go back to zero here, so the
-  // fused kernel that follows in the stream starts from a clean slate.
-  for (int i = threadIdx.x; i < num_clear; i += blockDim.x) clear_ptr[i] = 0u;
 
   for (int p = threadIdx.x; p < world; p += blockDim.x) {
     uint32_t* theirs = reinterpret_cast<uint32_t*>(peer_slots[p]) + rank;
@@ -90,11 +87,9 @@ extern "C" int ug_signal_wait(uint64_t counter, uint32_t expected, uint64_t stat
 }
 
 extern "C" int ug_signal_barrier(const uint64_t* peer_slots_dev, int world, int rank, uint64_t seq_counter,
-                                 uint64_t status, uint64_t timeout_ns, uint64_t clear_ptr, int num_clear,
-                                 void* stream) {
+                                 uint64_t status, uint64_t timeout_ns, void* stream) {
   if (world <= 0 || rank < 0 || rank >= world) return static_cast<int>(cudaErrorInvalidValue);
   signal_barrier_kernel<<<1, kBarrierThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      peer_slots_dev, world, rank, reinterpret_cast<uint32_t*>(seq_counter), reinterpret_cast<uint32_t*>(status), timeout_ns,
-      reinterpret_cast<uint32_t*>(clear_ptr), num_clear);
+      peer_slots_dev, world, rank, reinterpret_cast<uint32_t*>(seq_counter), reinterpret_cast<uint32_t*>(status), timeout_ns);
   return static_cast<int>(cudaGetLastError());
 }

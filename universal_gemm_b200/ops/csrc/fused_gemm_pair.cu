@@ -279,10 +279,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) ug_fused_gemm_pair_kernel(cons
     }
   } else {
     // ------------------------------------------------------------ fetch warps (and the epilogue warps at the start)
-    if (warp >= kFetchWarp0)
-      trace_fetch(P, blockIdx.x, lane, fetch_pieces(P, ctl, lane, 0u));
-    else if (P.fetch_helpers != 0)
-      trace_fetch(P, blockIdx.x, lane, fetch_pieces(P, ctl, lane, smem_u32(&sh->acc_full[0])));
+    trace_fetch(P, blockIdx.x, lane, fetch_pieces(P, ctl, lane, warp >= kFetchWarp0 ? 0u : smem_u32(&sh->acc_full[0])));
   }
   if (warp >= kEpiWarp0 && warp < kFetchWarp0) {
     // ------------------------------------------------------------ epilogue (both CTAs, own 128 rows)

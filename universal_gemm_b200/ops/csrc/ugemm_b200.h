@@ -102,7 +102,7 @@ typedef struct {
   uint64_t sched;            // 0 = static round-robin tiles; else a uint32, zero at launch (and put back to zero by the last
                              // worker to finish): the next tile claim, workers claim tiles dynamically
   int32_t fetch_depth;       // 16-byte loads a fetch-warp lane keeps in flight: 4, 8 or 16 (0 means 16)
-  int32_t fetch_helpers;     // 1: the epilogue warps copy pieces too until their first accumulator is complete
+  int32_t reserved0;
   uint64_t finished;         // 0, or a uint32 count of finished workers (CTAs, or CTA pairs), zero at launch: the last one puts
                              // back to zero what a launch expects there (this count, sched[0], the counters and the piece cursor)
   uint64_t part_flags;       // uint32 counters of the cut tiles (UgTask::part_flag), zero at launch, re-armed like the others
@@ -176,10 +176,8 @@ int ug_fused_gemm_smem_bytes(void);
 // this process) of rank p's counter array uint32[world]; the kernel advances the
 // local uint32 at `seq_counter`, adds 1 to slot `rank` of every peer and waits until
 // its own slots reach the new sequence number.
-// Also zeroes `num_clear` uint32 words at `clear_ptr` (plan flags) when non-zero.
 int ug_signal_barrier(const uint64_t* peer_slots_dev, int world, int rank, uint64_t seq_counter,
-                      uint64_t status, uint64_t timeout_ns, uint64_t clear_ptr, int num_clear,
-                      void* stream);
+                      uint64_t status, uint64_t timeout_ns, void* stream);
 // Point-to-point signals: add `value` to a uint32 counter (possibly in a peer's memory) after all earlier
 // work of the stream; wait (bounded) until a local counter has reached `expected`.
 int ug_signal_add(uint64_t counter, uint32_t value, void* stream);

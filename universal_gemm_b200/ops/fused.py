@@ -202,21 +202,20 @@ def _stream(raw: int, device: torch.device):
 class FusedProgram:
     """Device-resident tables of one lowered plan, ready to launch.
 
-    Launches of one program share its tables, staged copies, counters and workspace, so they run one after the other: a
+    A launch expects its counters at zero and leaves them there (the last worker to finish puts them back).  Launches of
+    one program share its tables, staged copies, counters and workspace, so they run one after the other: a
     launch on another stream than the last one waits for that one, and the memory is marked as used on every stream that
     launches it (it belongs to the stream it was built on, which would get it back while another still runs).  Replays of
     a graph that a caller captured cannot be seen from here: whoever replays it orders them."""
 
     def __init__(self, *, device: torch.device, tables: torch.Tensor, staging: torch.Tensor | None,
-                 workspace: torch.Tensor | None, params: native.FusedParams, grid: int, clear_ptr: int, num_clear: int, stats: dict):
+                 workspace: torch.Tensor | None, params: native.FusedParams, grid: int, stats: dict):
         self.device = device
         self._tables = tables
         self._staging = staging
         self._workspace = workspace
         self.params = params
         self.grid = grid
-        self.clear_ptr = clear_ptr
-        self.num_clear = num_clear
         self.stats = stats
         self._trace: torch.Tensor | None = None
         self._entry = native.lib().ug_fused_gemm_pair if params.cta_pair else native.lib().ug_fused_gemm
@@ -258,13 +257,6 @@ class FusedProgram:
 
     def set_status_ptr(self, ptr: int) -> None:
         self.params.status = ptr
-
-    def reset_flags(self, stream: int) -> None:
-        """Zero the chunk counters and the piece cursor (needed before every launch
-        when the program stages anything and no barrier kernel clears them)."""
-        if self.num_clear > 0:
-            native.check(native.lib().ug_zero_2d(self.clear_ptr, self.num_clear * 4, 1, self.num_clear * 4,
-                                                 ctypes.c_void_p(stream)), "ug_zero_2d(flags)")
 
     def launch(self, stream: int, checksum: int = 0) -> None:
         """Queue one launch on ``stream`` (the current stream); ``checksum``: address of the double it adds its sum to."""
@@ -805,7 +797,6 @@ class FusedProgramBuilder:
         remote_total = sum(st.src.remote_bytes() for st in staged.values() if st.pieces_of is None)
         need_gbs = remote_total / (modelled_us * 1e3) if modelled_us else float("inf")
         params.fetch_depth = int(os.environ.get("UGEMM_FETCH_DEPTH", "0")) or (8 if need_gbs < 300.0 else 16)
-        params.fetch_helpers = 1
         params.timeout_ns = self.timeout_ns
         stats = dict(tasks=len(task_rows), segments=len(seg_rows), tiles=total_tiles, maps=len(map_specs),
                      pieces=num_pieces, staged_bytes=staging_bytes, tile_m=variant if pair else BM,
@@ -816,7 +807,6 @@ class FusedProgramBuilder:
                      remote_bytes=sum(st.src.remote_bytes() for st in staged.values() if st.pieces_of is None),
                      grid=grid)
         prog = FusedProgram(device=dev, tables=tables, staging=staging, workspace=workspace, params=params, grid=grid,
-                            clear_ptr=0, num_clear=0,      # the kernel puts its counters back to zero itself
                             stats=stats)
         if workspace is not None:
             nbytes = workspace.numel() * 4

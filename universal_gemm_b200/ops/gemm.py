@@ -52,11 +52,7 @@ def build_gemm_program(a_parts: Sequence[torch.Tensor], b_parts: Sequence[torch.
 
 def run_program(prog: FusedProgram, device: torch.device) -> None:
     state = DeviceState.get(device)
-    stream = state.stream()
-    if prog.num_clear:
-        prog.reset_flags(stream)
-        state.launches += 1
-    prog.launch(stream)
+    prog.launch(state.stream())
     state.launches += 1
 
 

@@ -91,7 +91,7 @@ class FusedParams(ctypes.Structure):
         ("num_segs", c_int32), ("cta_pair", c_int32),
         ("trace", c_uint64), ("trace_slots", c_int32), ("epi_poll_ns", c_int32),
         ("sched", c_uint64),
-        ("fetch_depth", c_int32), ("fetch_helpers", c_int32),
+        ("fetch_depth", c_int32), ("reserved0", c_int32),
         ("finished", c_uint64), ("part_flags", c_uint64), ("num_part_flags", c_int32), ("claim_first", c_int32),
         ("checksum", c_uint64),
     ]
@@ -135,7 +135,7 @@ def lib() -> ctypes.CDLL:
     L.ug_fused_gemm_pair.argtypes = [POINTER(FusedParams), c_int, c_void_p]
     L.ug_fused_gemm_pair.restype = c_int
     L.ug_fused_gemm_pair_max_pairs.restype = c_int
-    L.ug_signal_barrier.argtypes = [c_uint64, c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int,
+    L.ug_signal_barrier.argtypes = [c_uint64, c_int, c_int, c_uint64, c_uint64, c_uint64,
                                     c_void_p]
     L.ug_zero_2d.argtypes = [c_uint64, c_int64, c_int32, c_int64, c_void_p]
     L.ug_signal_add.argtypes = [c_uint64, c_uint32, c_void_p]

@@ -228,13 +228,9 @@ def _run_fused(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequ
     if prof:
         e0, e1, e2, e3 = (torch.cuda.Event(enable_timing=True) for _ in range(4))
         e0.record()
-    # Entry barrier: every rank's operands (and zeroed C) are in place before any peer touches
-    # them; it also clears this plan's chunk counters.
-    if barriers or prog.num_clear:
-        if barriers:
-            world.device_barrier(prog.clear_ptr, prog.num_clear)
-        else:
-            state.zero_2d(prog.clear_ptr, prog.num_clear * 4, 1, prog.num_clear * 4)
+    # Entry barrier: every rank's operands (and zeroed C) are in place before any peer touches them.
+    if barriers:
+        world.device_barrier()
     if prof:
         e1.record()
     if checksum is not None:

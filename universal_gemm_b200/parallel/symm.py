@@ -142,7 +142,7 @@ class World:
         """Host-level barrier across the ranks (collective)."""
         raise NotImplementedError
 
-    def device_barrier(self, clear_ptr: int = 0, num_clear: int = 0) -> int:
+    def device_barrier(self) -> int:
         """Stream-ordered barrier across the ranks; returns the number of kernels launched."""
         raise NotImplementedError
 
@@ -305,11 +305,11 @@ class CudaIpcWorld(World):
     def barrier(self) -> None:
         self.comm.barrier()
 
-    def device_barrier(self, clear_ptr: int = 0, num_clear: int = 0) -> int:
+    def device_barrier(self) -> int:
         L = self._native.lib()
         self._native.check(
             L.ug_signal_barrier(self._slots.data_ptr(), self.size, self.rank, self._seq.data_ptr(),
-                                self.state.status_ptr, self.timeout_ns, clear_ptr, num_clear,
+                                self.state.status_ptr, self.timeout_ns,
                                 ctypes.c_void_p(self.state.stream())), "ug_signal_barrier")
         self.state.launches += 1
         return 1
@@ -403,7 +403,7 @@ class ShmWorld(World):
     def barrier(self) -> None:
         self.comm.barrier()
 
-    def device_barrier(self, clear_ptr: int = 0, num_clear: int = 0) -> int:
+    def device_barrier(self) -> int:
         self.barrier()
         return 0
 
@@ -479,14 +479,8 @@ class EmulatedWorld(World):
     def barrier(self) -> None:
         pass
 
-    def device_barrier(self, clear_ptr: int = 0, num_clear: int = 0) -> int:
-        # Ranks run one after the other, so only the local clearing part of the barrier remains.
-        if num_clear and self.is_cuda:
-            from ..ops.device import DeviceState
-
-            DeviceState.get(self.device).zero_2d(clear_ptr, num_clear * 4, 1, num_clear * 4)
-            return 1
-        return 0
+    def device_barrier(self) -> int:
+        return 0           # ranks run one after the other
 
 
 class SingleWorld(EmulatedWorld):
