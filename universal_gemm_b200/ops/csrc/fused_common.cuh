@@ -465,7 +465,6 @@ __device__ __forceinline__ void store_chunk_f32_ragged(float* sb, const uint32_t
   __syncwarp();
 }
 
-// Cut tiles, 64 x 16383 x 16383 (64 tiles on 148 SMs, two parts each): 104 us per call instead of 124 for whole pair tiles.
 // Sums of the other parts of a tile whose K blocks were cut (UgTask::part_count): `base` is this epilogue warp's block of
 // the first part: groups of four columns, in a group 16 bytes per row, so that a warp's access is four whole lines.
 struct Partials {
@@ -488,7 +487,8 @@ __device__ __forceinline__ void add_partial(uint32_t (&v)[32], const float4 (&x)
   }
 }
 // Add them to this warp's accumulator columns in place (TMEM), so that the drain that follows is the ordinary one.  Bound
-// by the latency of the reads (L2), a block of 4 KiB per warp at a time: a second one in registers would spill.
+// by the latency of the reads (L2), a block of 4 KiB per warp at a time: a second one in registers would spill.  Cut tiles as
+// a whole, 64 x 16383 x 16383 (64 tiles on 148 SMs, two parts each): 104 us per call, 124 with whole pair tiles.
 __device__ __forceinline__ void add_partials(uint32_t taddr, int n_rem, const Partials& pt, int lane) {
 #pragma unroll 1
   for (int c = 0; c < n_rem; c += 32) {
@@ -740,9 +740,9 @@ __device__ __forceinline__ void copy_flat_vec(const UgPiece& pc, int lane, int v
   }
 }
 
-// Copy one piece with the 32 lanes of a warp.  mode 0: 16-byte vectors, sixteen in
-// flight per lane.  mode 1: the source is only 2-byte aligned; every 16-byte
-// destination vector is gathered from eight 2-byte loads.
+// Copy one piece with the 32 lanes of a warp.  mode 0: 16-byte vectors, `depth` in flight per lane.  mode 1: the source is
+// only 2-byte aligned; every 16-byte destination vector is shifted out of the two aligned source vectors that cover it.
+// Modes 2 and 3: fp32 sources, split into two bf16 parts (copy_piece_split_f32), 16-byte aligned or not.
 __device__ __forceinline__ void copy_piece(const UgPiece& pc, int lane, int depth) {
   const int vec_per_row = (pc.row_bytes + 15) >> 4;
   if (vec_per_row <= 0) return;

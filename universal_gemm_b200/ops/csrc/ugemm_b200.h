@@ -43,7 +43,7 @@ typedef struct __attribute__((aligned(16))) {
   int32_t k_len;
   int32_t a_flag, b_flag;
   int32_t b_box;         // 64-column chunks of B per TMA load: 0 or 1 (2-D map), or all that a CTA needs of a tile (3-D map)
-  int32_t k_pos;         // K offset of this segment in its staged operands (0 when both are read in place)
+  int32_t k_pos;         // K offset of this segment in its operands' slices (names the K range of staged ones)
   int32_t a_step, b_step;   // counters per K range of the staged operand: chunk i of range r has counter flag + r * step + i
   int32_t pad[3];
 } UgSegment;  // 64 bytes
@@ -78,7 +78,8 @@ typedef struct __attribute__((aligned(16))) {
   int32_t rows;
   int32_t row_bytes;       // payload bytes per row
   int32_t flag;            // counter to bump when the piece has landed
-  int32_t mode;            // 0: 16-byte vectors (src 16 B aligned), 1: 2-byte elements (dst aligned, src arbitrary)
+  int32_t mode;            // low byte 0: bf16, src 16 B aligned; 1: bf16, src 2 B aligned; 2: fp32 split into two bf16 parts,
+                           // src 16 B aligned; 3: the same, src 4 B aligned.  2 and 3: the low parts go (mode >> 8) KiB past dst
 } UgPiece;  // 48 bytes
 
 typedef struct {

@@ -393,7 +393,8 @@ class FusedProgramBuilder:
         factor when C is a peer's memory.  Variants with double-buffered accumulators pay a part of the epilogue per
         tile (``drag``) and the last one in full, the others all of it.  A last, partly filled wave counts as it will
         run (:meth:`_choose_parts`).  Tiles are dealt round-robin to the workers (CTAs, or CTA pairs) as the
-        kernel does; the variant with the smallest busiest worker wins."""
+        kernel does; the variant with the smallest busiest worker wins.  The model knows no memory bandwidth: where an
+        operand streams (64 x 16383 x 16383: 65 us modelled, 83 for B alone) it ranks variants but is no estimate."""
         if self.tile_m is not None:
             return self.tile_m
         best = None
@@ -906,12 +907,15 @@ class FusedProgramBuilder:
         if len(blocks) != 1 or tail == 0 or any(t.tile_n != BN for t in tasks):
             return None
         if not v["hidden"] and any(t.c_remote for t in tasks):
-            return None                  # every part of such a tile would expose a drain, next to the exposed pushes
+            # every part of such a tile would expose a drain, next to the exposed pushes (reasoned, not measured: such
+            # plans take a variant with a hidden drain unless the caller names this one)
+            return None
         kb = blocks.pop()
         epi = self._epilogue_us(tasks[-1], v)
         tile = self._tile_us(kb, epi, v)
         whole = -(-total // workers) * tile
-        # what the launch takes without parts: the last wave's tiles at half width where that applies
+        # What the launch takes without parts: the last wave's tiles at half width where that applies.  Such a tile has half
+        # the tensor cycles and two thirds of the operand bytes; 0.7 of a tile time is taken between the two, not measured.
         plain = whole
         if total > workers and 2 * tail <= workers and self._split_tail(tasks, bm, workers) != tasks:
             plain = (total // workers + 0.7) * tile
@@ -943,6 +947,7 @@ class FusedProgramBuilder:
             end = max(end, lo + tile if rest else lo) + part_us * (p - 1)
             if best is None or end < best[0]:
                 best = (end, p)
+        # a cut has to win by 5 %, half of what the model is allowed to be off against measured kernels
         if best is None or best[0] + _CUT_US > 0.95 * plain:
             return 0, 1, whole - plain
         return tail, best[1], whole - best[0]
