@@ -260,20 +260,33 @@ class FusedProgram:
 
     def launch(self, stream: int, checksum: int = 0) -> None:
         """Queue one launch on ``stream`` (the current stream); ``checksum``: address of the double it adds its sum to."""
-        self.run_on(stream, self._call, stream, checksum)
+        self.begin(stream)
+        try:
+            self.call(stream, checksum)
+        finally:
+            self.end(stream)
 
-    def _call(self, stream: int, checksum: int) -> None:
+    def begin(self, stream: int) -> None:
+        """What is queued on ``stream``, the current one, from here to :meth:`end` runs after the program's earlier launches:
+        one :meth:`call` or the replay of a graph with one, and what belongs to it (the zeroing of C, the barrier)."""
+        self._lock.acquire()
+        if stream != self._last:
+            try:
+                self._change_stream(stream)
+            except BaseException:
+                self._lock.release()
+                raise
+
+    def call(self, stream: int, checksum: int = 0) -> None:
         self.params.checksum = checksum
         native.check(self._entry(self._params_ref, self.grid, stream), "ug_fused_gemm")
 
-    def run_on(self, stream: int, queue: Callable, *args) -> None:
-        """``queue(*args)`` puts a launch of this program (or the replay of a graph with one) on ``stream``, the current one."""
-        with self._lock:
-            if stream != self._last:
-                self._change_stream(stream)
-            queue(*args)
+    def end(self, stream: int) -> None:
+        try:
             if stream:
                 self._mark()
+        finally:
+            self._lock.release()
 
     def _mark(self) -> None:
         if torch.cuda.is_current_stream_capturing():

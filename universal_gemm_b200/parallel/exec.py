@@ -221,22 +221,26 @@ def _run_fused(kind: str, a: DistMatrix, b: DistMatrix, c: DistMatrix, ops: Sequ
     world = c.world
     state = DeviceState.get(c.device)
     prog, needs_zero = program or _program(kind, a, b, c, ops, fuse_replica_reduce, beta, gelu_out)
-    if needs_zero:        # several ranks add into C: clear it before the entry barrier lets anyone push
-        pad = c.local_padded
-        state.zero_2d(pad.data_ptr(), c.ld * c.itemsize, pad.shape[0], c.ld * c.itemsize)
+    if checksum is not None and (checksum.dtype != torch.float64 or checksum.numel() < 1 or checksum.device != c.device):
+        raise ValueError("checksum must be a float64 tensor on the device of C")
     prof = profile.enabled
-    if prof:
-        e0, e1, e2, e3 = (torch.cuda.Event(enable_timing=True) for _ in range(4))
-        e0.record()
-    # Entry barrier: every rank's operands (and zeroed C) are in place before any peer touches them.
-    if barriers:
-        world.device_barrier()
-    if prof:
-        e1.record()
-    if checksum is not None:
-        if checksum.dtype != torch.float64 or checksum.numel() < 1 or checksum.device != c.device:
-            raise ValueError("checksum must be a float64 tensor on the device of C")
-    prog.launch(state.stream(), checksum.data_ptr() if checksum is not None else 0)
+    stream = state.stream()
+    prog.begin(stream)
+    try:
+        if needs_zero:    # several ranks add into C: clear it before the entry barrier lets anyone push
+            pad = c.local_padded
+            state.zero_2d(pad.data_ptr(), c.ld * c.itemsize, pad.shape[0], c.ld * c.itemsize)
+        if prof:
+            e0, e1, e2, e3 = (torch.cuda.Event(enable_timing=True) for _ in range(4))
+            e0.record()
+        # Entry barrier: every rank's operands (and zeroed C) are in place before any peer touches them.
+        if barriers:
+            world.device_barrier()
+        if prof:
+            e1.record()
+        prog.call(stream, checksum.data_ptr() if checksum is not None else 0)
+    finally:
+        prog.end(stream)
     state.launches += 1
     if prof:
         e2.record()

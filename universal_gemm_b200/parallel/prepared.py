@@ -47,7 +47,12 @@ class MatmulPlan:
     def run(self) -> None:
         """Queue one ``C (+)= A @ B`` on the current stream."""
         if self._graph is not None:
-            self.program.run_on(DeviceState.get(self.c.device).stream(), self._graph.replay)
+            stream = DeviceState.get(self.c.device).stream()
+            self.program.begin(stream)
+            try:
+                self._graph.replay()
+            finally:
+                self.program.end(stream)
             return
         self._launch()
 
