@@ -252,6 +252,9 @@ def test_workspaces_of_all_programs_are_bounded(monkeypatch):
         return b._choose_parts(b.tasks, 128)[1]
 
     assert parts() == 2
+    long_k = FusedProgramBuilder("cpu", num_sms=148)     # 88 tiles of 256 x 256 in five parts: 88 MiB
+    long_k.add_task(_task(2048, 12288, 49152))
+    assert long_k._choose_parts(long_k.tasks, 256)[:2] == (88, 5)
     monkeypatch.setitem(fused._workspace_bytes, None, fused._MAX_WORKSPACE_BYTES - (8 << 20))
     assert parts() == 2
     monkeypatch.setitem(fused._workspace_bytes, None, fused._MAX_WORKSPACE_BYTES - (8 << 20) + 1)

@@ -939,9 +939,9 @@ class FusedProgramBuilder:
         full, rest = divmod(total - tail, workers)
         part_us = v["part_us"] * min(1.0, max(t.m for t in tasks) / bm)     # only rows that exist are read
         best = None
-        room = min(_MAX_PART_BYTES, _MAX_WORKSPACE_BYTES - _workspace_bytes.get(self.device.index, 0))
+        most_bytes = min(_MAX_PART_BYTES, _MAX_WORKSPACE_BYTES - _workspace_bytes.get(self.device.index, 0))
         for p in range(2, _MAX_PARTS + 1):
-            if kb // p < 4 or tail * (p - 1) * bm * BN * 4 > room:
+            if kb // p < 4 or tail * (p - 1) * bm * BN * 4 > most_bytes:
                 break
             part = self._tile_us(-(-kb // p), epi, v)
             # greedy: `workers - rest` workers are free after `full` tiles, `rest` one tile later
