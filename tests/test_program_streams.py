@@ -263,3 +263,67 @@ def test_counters_are_back_at_zero_after_a_launch_that_gave_up(tile_m):
     assert _zero_counters(prog)
     want = a.double() @ b.double()
     assert (c.double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["stationary_b", "stationary_c"])
+@pytest.mark.parametrize("triple", [("row", "column", "row"), ("block", "row", "column"), ("column", "block", "block")])
+@pytest.mark.parametrize("tile_m", ["128", "256", "pair"])
+@pytest.mark.parametrize("c_dtype", [torch.float32, torch.bfloat16])
+def test_cut_tiles_on_several_ranks_stay_inside_their_allocations(method, triple, tile_m, c_dtype, monkeypatch):
+    """Every tile of every rank in three K parts, through ug.matmul: operands staged from peers in several K ranges, results
+    pushed into peers; guard regions around every tile."""
+    from helpers import build_cluster_matrices
+    from universal_gemm_b200.parallel import exec as X
+
+    builder = fused.FusedProgramBuilder
+    monkeypatch.setattr(fused, "FusedProgramBuilder", lambda *args, **kw: builder(*args, **dict(kw, split_k=False, parts=3)))
+    monkeypatch.setenv("UGEMM_TILE_M", tile_m)
+    m, n, k = 301, 403, 1900
+    full_a, full_b, full_c = make_inputs(m, n, k, seed=21, device=_dev())
+    cluster = ug.EmulatedCluster(4, _dev(), guard_bytes=4096)
+    mats = build_cluster_matrices(cluster, full_a, full_b, full_c, triple, 1, torch.bfloat16, c_dtype)
+    X.clear_program_cache()
+    for a, b, c in mats:
+        ug.matmul(a, b, c, method=method)
+    ug.check_status(_dev())
+    assert cluster.check_guards() == 12
+    progs = [p for _, p in X.cached_programs()]
+    assert progs and all(p.stats["parts"] == 3 and p.stats["cut_tiles"] > 0 for p in progs)
+    want = full_c.to(c_dtype).double() + full_a.bfloat16().double() @ full_b.bfloat16().double()
+    # bf16: as many roundings of a sum of two as ranks add into an element (four), 2^-8 each for the share and the result
+    tol = 1e-4 if c_dtype == torch.float32 else 4 * 2.0 ** -8
+    assert ((mats[0][2].full_tensor().double() - want).abs() <= tol * (1.0 + want.abs())).all()
+    X.clear_program_cache()
+
+
+@pytest.mark.gpu
+def test_matrices_made_again_at_old_addresses():
+    """Clusters made and dropped in turn, of both result types and with one matrix kept over: every call runs a program of
+    its own matrices, and the dropped ones' programs are gone."""
+    import gc
+
+    from helpers import build_cluster_matrices
+    from universal_gemm_b200.parallel import exec as X
+
+    m, n, k = 301, 403, 700
+    full_a, full_b, full_c = make_inputs(m, n, k, seed=22, device=_dev())
+    prod = full_a.bfloat16().double() @ full_b.bfloat16().double()
+    X.clear_program_cache()
+    kept = []
+    for i in range(12):
+        cluster = ug.EmulatedCluster(2 + 2 * (i % 2), _dev())
+        dtype = (torch.float32, torch.bfloat16)[i // 2 % 2]
+        mats = build_cluster_matrices(cluster, full_a, full_b, full_c, ("block", "row", "column"), 1, torch.bfloat16, dtype)
+        if i % 3 == 1:                                       # peers' tiles move, this rank's may not
+            kept = [torch.empty(mats[0][0].nbytes, dtype=torch.uint8, device=_dev()) for _ in range(i)]
+        for a, b, c in mats:
+            ug.matmul(a, b, c, method="stationary_c")
+        ug.check_status(_dev())
+        want = full_c.to(dtype).double() + prod
+        tol = 1e-4 if dtype == torch.float32 else 2 * 2.0 ** -8
+        assert ((mats[0][2].full_tensor().double() - want).abs() <= tol * (1.0 + want.abs())).all()
+        assert len(X.cached_programs()) == len(mats)
+        del cluster, mats, a, b, c
+        gc.collect()
+        assert not X.cached_programs()
