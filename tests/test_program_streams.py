@@ -276,8 +276,9 @@ def test_cut_tiles_on_several_ranks_stay_inside_their_allocations(method, triple
     from helpers import build_cluster_matrices
     from universal_gemm_b200.parallel import exec as X
 
-    builder = fused.FusedProgramBuilder
-    monkeypatch.setattr(fused, "FusedProgramBuilder", lambda *args, **kw: builder(*args, **dict(kw, split_k=False, parts=3)))
+    init = fused.FusedProgramBuilder.__init__
+    monkeypatch.setattr(fused.FusedProgramBuilder, "__init__",
+                        lambda self, *args, **kw: init(self, *args, **dict(kw, split_k=False, parts=3)))
     monkeypatch.setenv("UGEMM_TILE_M", tile_m)
     m, n, k = 301, 403, 1900
     full_a, full_b, full_c = make_inputs(m, n, k, seed=21, device=_dev())
