@@ -343,6 +343,9 @@ class FusedProgramBuilder:
         if tile_m not in (None, 128, 256, "pair", "pair512"):
             raise ValueError('tile_m must be 128, 256, "pair" or "pair512"')
         self.tile_m = tile_m
+        self.env_tail_split = os.environ.get("UGEMM_TAIL_SPLIT", "1") != "0"
+        self.env_split_k = os.environ.get("UGEMM_SPLIT_K", "1") != "0"
+        self.env_dynamic = os.environ.get("UGEMM_DYNAMIC_TILES", "")
         self.tasks: list[TaskSpec] = []
         self._models: dict = {}      # variant -> (microseconds, cut) of the tasks so far
 
@@ -437,7 +440,7 @@ class FusedProgramBuilder:
         tile = 0
         last = 0.0
         tasks = self.tasks
-        if self.split_k and os.environ.get("UGEMM_SPLIT_K", "1") != "0":
+        if self.split_k and self.env_split_k:
             tasks = self._split_k([t if v["cols"] == BN else self._with_tile_n(t, v["cols"]) for t in tasks],
                                   v["rows"], workers)
         for t in tasks:
@@ -483,9 +486,9 @@ class FusedProgramBuilder:
         modelled_us, cut = self._model(variant)
         if cut is not None and cut[1] > 1:
             tasks = self._cut_parts(tasks, BM, cut[0], cut[1])
-        elif os.environ.get("UGEMM_TAIL_SPLIT", "1") != "0":
+        elif self.env_tail_split:
             tasks = self._split_tail(tasks, BM, workers, 2 * BN if wide else BN)
-        if self.split_k and os.environ.get("UGEMM_SPLIT_K", "1") != "0":
+        if self.split_k and self.env_split_k:
             whole = tasks
             tasks = self._split_k(tasks, BM, workers)
             if len(tasks) > len(whole) and all(a.split for t in whole for a, _ in t.segments):
@@ -733,13 +736,15 @@ class FusedProgramBuilder:
                     row["part_ptr"] = workspace.data_ptr() + 4 * row["part_ptr"]
         seg_arr = np.zeros(max(len(seg_rows), 1), dtype=native.SEGMENT_DTYPE)
         for i, row in enumerate(seg_rows):
+            entry = seg_arr[i]
             for k, v in row.items():
-                seg_arr[i][k] = v
+                entry[k] = v
         task_arr = np.zeros(max(len(task_rows), 1), dtype=native.TASK_DTYPE)
         for i, row in enumerate(task_rows):
+            entry = task_arr[i]
             for k, v in row.items():
                 if k not in ("tile_n", "row_tab_at"):
-                    task_arr[i][k] = v
+                    entry[k] = v
         piece_arr = np.concatenate(ordered) if ordered else np.zeros(1, dtype=native.PIECE_DTYPE)
         num_pieces = len(piece_arr) if ordered else 0
         maps_blob = bytearray()
@@ -752,25 +757,22 @@ class FusedProgramBuilder:
         if not maps_blob:
             maps_blob = bytearray(128)
 
-        def pad(b: bytes, align: int = 256) -> bytes:
-            return b + bytes((-len(b)) % align)
-
         row_tab_arr = np.asarray(row_table or [0], dtype=np.uint64)
-        lengths = [len(pad(bytes(x))) for x in (maps_blob, task_arr.tobytes(), seg_arr.tobytes(), piece_arr.tobytes(),
-                                                flag_need.tobytes(), bytes(4 * (num_flags + 2)), bytes(8),
-                                                row_tab_arr.tobytes(), bytes(4 * max(num_part_flags, 1)))]
-        offsets = np.cumsum([0] + lengths)
-        tables = torch.empty(int(offsets[-1]) + 256, dtype=torch.uint8, device=dev)
+        offsets = [0]                # of the sections, 256-byte aligned each
+        for nbytes in (len(maps_blob), task_arr.nbytes, seg_arr.nbytes, piece_arr.nbytes, flag_need.nbytes, 4 * (num_flags + 2), 8,
+                       row_tab_arr.nbytes, 4 * max(num_part_flags, 1)):
+            offsets.append(offsets[-1] + _round_up(nbytes, 256))
+        tables = torch.empty(offsets[-1] + 256, dtype=torch.uint8, device=dev)
         base = _round_up(tables.data_ptr(), 256)
         shift = base - tables.data_ptr()
         for i, row in enumerate(task_rows):          # tasks with a row table point at their part of it
             if row["row_tab_at"] >= 0:
                 task_arr[i]["c_ptr"] = base + int(offsets[7]) + 8 * row["row_tab_at"]
                 task_arr[i]["ldc"] = 0
-        sections = [pad(bytes(maps_blob)), pad(task_arr.tobytes()), pad(seg_arr.tobytes()), pad(piece_arr.tobytes()),
-                    pad(flag_need.tobytes()), pad(bytes(4 * (num_flags + 2))), pad(bytes(8)), pad(row_tab_arr.tobytes()),
-                    pad(bytes(4 * max(num_part_flags, 1)))]
-        blob = np.frombuffer(b"".join(sections), dtype=np.uint8).copy()
+        blob = np.zeros(offsets[-1], dtype=np.uint8)
+        for section, data in ((0, np.frombuffer(maps_blob, dtype=np.uint8)), (1, task_arr), (2, seg_arr), (3, piece_arr), (4, flag_need),
+                              (7, row_tab_arr)):             # the others are counters: zero
+            blob[offsets[section]:offsets[section] + data.nbytes] = data.view(np.uint8)
         tables[shift:shift + len(blob)].copy_(torch.from_numpy(blob))
 
         params = native.FusedParams()
@@ -794,10 +796,9 @@ class FusedProgramBuilder:
         # variants, where it measured +6-9 % on the headline GEMM (workers finish 90 us apart instead of 450 us); off
         # for the one-CTA variants, where it measured level: under the power cap the SMs that finish early leave their
         # share of the power budget to the others.  UGEMM_DYNAMIC_TILES=0 / 1 overrides.
-        dyn_env = os.environ.get("UGEMM_DYNAMIC_TILES", "")
         # Cut tiles need it, from the first tile on: a part then only ever waits for parts claimed before it by workers
         # that run, also when other work keeps some of this launch's CTAs from starting.
-        dynamic = num_part_flags > 0 or (pair if dyn_env == "" else dyn_env != "0")
+        dynamic = num_part_flags > 0 or (pair if self.env_dynamic == "" else self.env_dynamic != "0")
         params.claim_first = 1 if num_part_flags else 0
         params.part_flags = base + int(offsets[8])
         params.num_part_flags = num_part_flags
@@ -907,12 +908,12 @@ class FusedProgramBuilder:
         v = _VARIANTS[variant]
         workers = self.num_sms // 2 if v["pair"] else self.num_sms
         if self.parts == 1 or self.split_k or workers < 1 or v["cols"] != BN or not tasks \
-                or os.environ.get("UGEMM_TAIL_SPLIT", "1") == "0":
+                or not self.env_tail_split:
             return None
         bm = v["rows"]
         counts = [((t.m + bm - 1) // bm) * ((t.n + BN - 1) // BN) for t in tasks]
         total = sum(counts)
-        claimed = os.environ.get("UGEMM_DYNAMIC_TILES", "") != "0"       # without claims a part might wait for a part behind it
+        claimed = self.env_dynamic != "0"       # without claims a part might wait for a part behind it
         if self.parts is not None:
             return (total, self.parts, 0.0) if claimed and min(t.total_blocks() for t in tasks) >= self.parts else None
         blocks = {t.total_blocks() for t in tasks}
@@ -947,6 +948,9 @@ class FusedProgramBuilder:
             # greedy: `workers - rest` workers are free after `full` tiles, `rest` one tile later
             lo = full * tile
             need, end = tail * p, None
+            bound = lo + -(-need // workers) * part + part_us * (p - 1)      # all workers together are no faster
+            if bound + _CUT_US > 0.95 * plain or (best is not None and bound >= best[0]):
+                continue
             for i in range(1, need + 1):
                 for t in ((lo + i * part), (lo + tile + i * part) if rest else (lo + i * part)):
                     room = int((t - lo) / part + 1e-6) * (workers - rest)
@@ -960,7 +964,7 @@ class FusedProgramBuilder:
             end = max(end, lo + tile if rest else lo) + part_us * (p - 1)
             if best is None or end < best[0]:
                 best = (end, p)
-        # a cut has to win by 5 %, half of what the model is allowed to be off against measured kernels
+        # a cut has to win by 5 % (here and above), half of what the model is allowed to be off against measured kernels
         if best is None or best[0] + _CUT_US > 0.95 * plain:
             return 0, 1, whole - plain
         return tail, best[1], whole - best[0]
