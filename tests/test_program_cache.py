@@ -90,6 +90,18 @@ def test_a_program_goes_with_the_first_of_its_matrices(which, lowered):
     assert _get(*other) is keep
 
 
+def test_a_weight_remembers_only_the_programs_that_are_left():
+    """A loop over new inputs and results with one weight: nothing of the earlier calls stays."""
+    a, b, c = _triple([1 << 20, 2 << 20])
+    _get(a, b, c)
+    for i in range(5):
+        x, _, y = _triple([(3 + i) << 20, 2 << 20])
+        _get(x, b, y)
+        del x, y
+        gc.collect()
+        assert len(X._program_cache) == 1 and len(X._programs_of[b.buffer.uid]) == 1
+
+
 def test_freeing_a_matrix_drops_its_programs_only():
     a, b, c = _triple([1 << 20, 2 << 20])
     other = _triple([3 << 20, 4 << 20])

@@ -52,6 +52,10 @@ def drop_programs_for(uid: int) -> None:
     when a matrix is freed, and when its buffer is collected)."""
     for key in list(_programs_of.pop(uid, ())):
         _program_cache.pop(key, None)
+        for other in (*key[1:4], key[7]):          # a weight outlives the inputs and results it was used with
+            keys = _programs_of.get(other)
+            if keys is not None:
+                keys.discard(key)
 
 
 def _keep_program(key: tuple, entry: tuple, buffers: Sequence[Any]) -> None:
